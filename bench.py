@@ -1222,10 +1222,9 @@ def c2_line(args, workload_name, world=1, barrier=lambda: None, cpu_substeps=Non
     n_chunks = len(frame_chunks(kw["frame_dt"], kw["dt"]))
     per_substep = 2 + kw["constraints_iter"] * (3 + (1 if scatter == "gather" else 0))
     launches_per_frame = n_chunks * kw["substeps_num"] * per_substep
-    # a body whose patches are all resident (three per SM) takes one launch per chunk
-    # outside the profiled frames
-    resident = (scatter == "patch" and tpt == 2 and not pipe and not args.patch_reduce and
-                solver._n_patches <= 3 * torch.cuda.get_device_properties(0).multi_processor_count)
+    # a body whose patches are all resident takes one launch per chunk outside the
+    # profiled frames
+    resident = solver.launch_info()["form"] != 0
     flush = torch.empty(L2_FLUSH_BYTES // 4, dtype=torch.float32, device="cuda")
     stream = torch.cuda.current_stream()
 

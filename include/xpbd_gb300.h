@@ -252,6 +252,21 @@ enum xpbd_kernel_class {
  * solve_step, neohookean_solver.py:454-560.) */
 int xpbd_set_profiling(void* handle, int32_t enable);
 
+/* How the next frame's substeps run with the parameters in force.  form 0: one
+ * launch per phase of every Jacobi iteration; 1: whole substeps in one launch,
+ * a thread-block cluster per body; 2: the same as one cooperative grid with a
+ * CTA per patch.  Forms 1 and 2 are those of bodies small enough to stay on
+ * the SMs; while profiling is on, such a body takes form 0, whose phases
+ * the profile brackets.  No counterpart in the reference. */
+typedef struct xpbd_launch_info {
+  int32_t form;
+  int32_t ctas;            /* forms 1 and 2: CTAs of the launch */
+  int32_t patches_per_cta; /* forms 1 and 2: 1 or 2 */
+  int32_t rounds;          /* form 1: the clusters over those resident at once, rounded up */
+  int64_t overlapped;      /* launches issued or captured so far that may start while the one before drains */
+} xpbd_launch_info;
+int xpbd_get_launch_info(void* handle, xpbd_launch_info* out);
+
 /* L2 eviction policy of the read-only tet records in the tile (PATCH)
  * sweeps.  mode -1: automatic, the default: evict_last when the records and
  * the per-iteration state fit in 80% of the device's L2, else plain loads;
@@ -474,6 +489,7 @@ int xpbd_batch_read_iterations(void* handle, int32_t* host_out, int32_t n, void*
 int xpbd_batch_get_rho_hat(void* handle, double* host_out, void* stream);
 
 int xpbd_batch_check_status(void* handle, void* stream);
+int xpbd_batch_get_launch_info(void* handle, xpbd_launch_info* out);
 int xpbd_batch_import_vec3(void* handle, int32_t field, const float* src, void* stream);
 int xpbd_batch_export_vec3(void* handle, int32_t field, float* dst, void* stream);
 int xpbd_batch_set_profiling(void* handle, int32_t enable);

@@ -96,6 +96,14 @@ class XpbdAdjoint(ctypes.Structure):
                 ("work_res_tet", _P)]
 
 
+class XpbdLaunchInfo(ctypes.Structure):
+    _fields_ = [("form", ctypes.c_int32), ("ctas", ctypes.c_int32), ("patches_per_cta", ctypes.c_int32),
+                ("rounds", ctypes.c_int32), ("overlapped", ctypes.c_int64)]
+
+    def as_dict(self):
+        return {k: getattr(self, k) for k, _ in self._fields_}
+
+
 # name -> (restype, argtypes); every symbol declared in include/xpbd_gb300.h
 _SIGNATURES = {
     "xpbd_abi_version": (ctypes.c_int, []),
@@ -123,6 +131,7 @@ _SIGNATURES = {
     "xpbd_import_vec3": (ctypes.c_int, [_P, ctypes.c_int32, _P, _P]),
     "xpbd_export_vec3": (ctypes.c_int, [_P, ctypes.c_int32, _P, _P]),
     "xpbd_check_status": (ctypes.c_int, [_P, _P]),
+    "xpbd_get_launch_info": (ctypes.c_int, [_P, ctypes.POINTER(XpbdLaunchInfo)]),
     "xpbd_save_rho_hat": (ctypes.c_int, [_P, _P, _P]),
     "xpbd_load_rho_hat": (ctypes.c_int, [_P, _P, _P]),
     "xpbd_substep_tape": (ctypes.c_int, [_P, ctypes.c_float, ctypes.POINTER(XpbdTape), _P]),
@@ -148,6 +157,7 @@ _SIGNATURES = {
     "xpbd_batch_read_iterations": (ctypes.c_int, [_P, _P, ctypes.c_int32, _P]),
     "xpbd_batch_get_rho_hat": (ctypes.c_int, [_P, _P, _P]),
     "xpbd_batch_check_status": (ctypes.c_int, [_P, _P]),
+    "xpbd_batch_get_launch_info": (ctypes.c_int, [_P, ctypes.POINTER(XpbdLaunchInfo)]),
     "xpbd_batch_import_vec3": (ctypes.c_int, [_P, ctypes.c_int32, _P, _P]),
     "xpbd_batch_export_vec3": (ctypes.c_int, [_P, ctypes.c_int32, _P, _P]),
     "xpbd_batch_set_profiling": (ctypes.c_int, [_P, ctypes.c_int32]),

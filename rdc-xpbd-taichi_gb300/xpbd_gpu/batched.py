@@ -433,7 +433,15 @@ class XPBDBatchedSolver:
         self.check_status()
         return a.elapsed_time(b) / reps
 
+    def launch_info(self):
+        """How the next frame runs (XPBDNeoHookeanSolver.launch_info)."""
+        out = _native.XpbdLaunchInfo()
+        _native.check(self._lib.xpbd_batch_get_launch_info(self._handle, _native.ctypes.byref(out)), batch=True)
+        return out.as_dict()
+
     def set_profiling(self, enable):
+        """Bracket every kernel launch with CUDA events.  A batch whose substeps are
+        single launches (launch_info) runs one launch per phase while profiled."""
         _native.check(self._lib.xpbd_batch_set_profiling(self._handle, 1 if enable else 0), batch=True)
 
     def read_profile(self, reset=False):

@@ -312,9 +312,20 @@ class XPBDNeoHookeanSolver(XPBDSolverBase):
                 self._stream()))
         return out
 
+    def launch_info(self):
+        """How the next frame runs: {'form': 0 one launch per phase, 1 whole substeps
+        in one launch (clusters), 2 the same (cooperative grid), 'ctas',
+        'patches_per_cta', 'rounds', 'overlapped'} (xpbd_launch_info)."""
+        self._sync()
+        out = _native.XpbdLaunchInfo()
+        _native.check(self._lib.xpbd_get_launch_info(self._handle, _native.ctypes.byref(out)))
+        return out.as_dict()
+
     def set_profiling(self, enable):
         """Bracket every kernel launch with CUDA events (with use_graph the
-        frame graph carries them as event record nodes)."""
+        frame graph carries them as event record nodes).  A body whose substeps
+        are single launches (launch_info) runs one launch per phase while
+        profiled: the profile is that of this other form, not of its frames."""
         _native.check(self._lib.xpbd_set_profiling(self._handle, 1 if enable else 0))
 
     def set_l2_hint(self, mode=-1):
