@@ -85,3 +85,16 @@ def test_form_of_a_body_with_per_tet_materials(dims, form):
     sim = DiffSim(m, _sdfs(), np.full(m.n_tets, np.log(1e5)), np.full(m.n_tets, 0.4), density=1000.0, use_graphs=False,
                   scatter="gather", **_kw())
     assert _form(sim.solver)[0] == 0
+
+
+@pytest.mark.parametrize("dims", [(4, 4, 4), (18, 18, 20), (19, 18, 19), (22, 22, 22)])
+@pytest.mark.parametrize("graph", [True, False])
+def test_gather_overlaps_the_projection_up_to_one_cta_per_sm(dims, graph):
+    """Every kernel of an iteration but the substep's first may overlap the one
+    before; the gather only where the projection leaves the SMs room."""
+    import torch
+    s = _solver(_mesh(dims), scatter="gather", substeps_num=1, use_graph=graph)
+    small = -(-s.n_tets // 256) <= torch.cuda.get_device_properties(0).multi_processor_count
+    assert small == (dims in ((4, 4, 4), (18, 18, 20)))
+    s.solve()
+    assert s.launch_info()["overlapped"] == (4 if small else 3) * 9 - 1
