@@ -98,3 +98,30 @@ def test_gather_overlaps_the_projection_up_to_one_cta_per_sm(dims, graph):
     assert small == (dims in ((4, 4, 4), (18, 18, 20)))
     s.solve()
     assert s.launch_info()["overlapped"] == (4 if small else 3) * 9 - 1
+
+
+@pytest.mark.parametrize("kind", ["gather", "atomic", "patch", "gradient", "gradient over the gather", "batch"])
+def test_the_switch_turns_every_overlap_off(kind, monkeypatch):
+    """XPBD_NO_PDL=1 when the solver is made: no launch overlaps, whatever layouts it has."""
+    import torch
+    from xpbd_gpu.batched import Body, XPBDBatchedSolver
+    from xpbd_gpu.differentiable import DiffSim, xpbd_simulate
+    counts = []
+    for off in ("0", "1"):
+        monkeypatch.setenv("XPBD_NO_PDL", off)
+        m = _mesh((9, 9, 9) if "gradient" in kind else (28, 26, 27))
+        if "gradient" in kind:
+            sim = DiffSim(m, _sdfs(), np.full(m.n_tets, np.log(1e5)), np.full(m.n_tets, 0.4), density=1000.0,
+                          use_graphs=False, scatter="gather" if "gather" in kind else "atomic", **_kw())
+            t = [torch.tensor(a, dtype=torch.float32, device="cuda", requires_grad=True)
+                 for a in (m.points, np.zeros_like(m.points), np.full(m.n_tets, np.log(1e5)), np.full(m.n_tets, 0.4))]
+            (xpbd_simulate(sim, *t, 1) ** 2).sum().backward()
+            s = sim.solver
+        elif kind == "batch":
+            s = XPBDBatchedSolver([Body(m, young_modulus=2e5, poisson_ratio=0.4, density=1000.0)], _sdfs(), **_kw())
+            s.solve()
+        else:
+            s = _solver(m, scatter=kind)
+            s.solve()
+        counts.append(s.launch_info()["overlapped"])
+    assert counts[0] > 0 and counts[1] == 0
