@@ -285,7 +285,9 @@ int xpbd_save_rho_hat(void* handle, double* dst_device, void* stream);
 int xpbd_load_rho_hat(void* handle, const double* src_device, void* stream);
 
 /* Sticky device error flags (XPBD_OK, XPBD_ERR_NONFINITE or XPBD_ERR_TIMEOUT);
- * synchronises. */
+ * synchronises.  TIMEOUT: a bounded wait of a kernel ran out (after about a
+ * second); the state is invalid, and later launches of form 2 return at
+ * once. */
 int xpbd_check_status(void* handle, void* stream);
 
 /* ------------------------------------------------------------------------
