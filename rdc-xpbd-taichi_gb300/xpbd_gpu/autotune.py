@@ -157,7 +157,11 @@ def tune_single(solver_cls, ctor_args, warmup=2, reps=5, cache=True, log=None):
     cands = single_candidates(per_tet)
     groups = {}
     for c in cands:
-        layout = ("patch", c[1]) if c[0] == "patch" else ("csr", 0)
+        layout = ("patch", c[1]) if c[0] == "patch" else ("gather", 0)
+        if per_tet and c[0] == "atomic":
+            # built as "atomic", such a body also has the patch layout, and a small one
+            # runs whole substeps in one launch
+            layout = ("atomic", 0)
         groups.setdefault(layout, []).append(c)
     sub_dt = float(ctor_args.get("dt", 1e-2)) / max(1, int(ctor_args.get("substeps_num", 1)))
     sub_dt = min(sub_dt, float(ctor_args.get("frame_dt", sub_dt)))
@@ -167,7 +171,7 @@ def tune_single(solver_cls, ctor_args, warmup=2, reps=5, cache=True, log=None):
         kw = dict(ctor_args)
         # candidates are timed at the fixed iteration count (stop mode off), so
         # that every replay does the same work
-        kw.update(scatter="gather" if layout[0] == "csr" else "patch", patch_tets=first[1] or 256,
+        kw.update(scatter=layout[0], patch_tets=first[1] or 256,
                   tets_per_thread=first[2], patch_pipeline=first[3], use_graph=True, monitor_convergence=False,
                   target_rel_residual=0.0, residual_floor=0.0)
         try:

@@ -42,3 +42,35 @@ def test_candidates_respect_per_tet_materials():
 def test_cache_path_env(monkeypatch, tmp_path):
     monkeypatch.setenv("XPBD_AUTOTUNE_CACHE", str(tmp_path / "x.json"))
     assert autotune.cache_path() == str(tmp_path / "x.json")
+
+
+class _Body:
+    """Stands in for the solver: what a layout's candidates are timed on."""
+    built = []
+
+    def __init__(self, scatter, patch_tets, **kw):
+        self.scatter, self._patch_tets = scatter, patch_tets
+        self.built_as = scatter
+        _Body.built.append(scatter)
+
+
+def _tune(monkeypatch, **kw):
+    from xpbd_gpu.mesh import kuhn_grid
+    timed = []
+    _Body.built = []
+    monkeypatch.setattr(autotune, "device_stamp", lambda device_index=None: "fake")
+    monkeypatch.setattr(autotune, "_time_graph_substeps",
+                        lambda s, dt, warmup, reps: timed.append((s.scatter, s.built_as)) or 1.0 + len(timed))
+    autotune.tune_single(_Body, dict(rest_pose=kuhn_grid(1, 1, 1, 1.0), **kw), cache=False)
+    return timed
+
+
+def test_per_tet_candidates_are_timed_as_they_would_be_built(monkeypatch):
+    """A solver built with scatter="atomic" and per-tet materials has a layout (and,
+    if small, a form) that one built with "gather" has not."""
+    import numpy as np
+    timed = _tune(monkeypatch, tet_young_modulus=np.ones(6))
+    assert sorted(timed) == [("atomic", "atomic"), ("gather", "gather")]
+    timed = _tune(monkeypatch)
+    assert ("atomic", "gather") in timed and ("gather", "gather") in timed  # one layout: switched in place
+    assert all(as_ == "patch" for s, as_ in timed if s == "patch")

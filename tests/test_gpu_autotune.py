@@ -64,3 +64,23 @@ def test_batch_autotune_restores_state(tmp_path):
     for sl in tuned.body_vert_slices:
         diag = float(np.linalg.norm(Y[sl].max(0) - Y[sl].min(0)))
         assert np.abs(X[sl] - Y[sl]).max() <= 1e-4 * diag
+
+
+def test_per_tet_body_is_timed_in_the_form_it_would_run(tmp_path, monkeypatch):
+    from xpbd_gpu import autotune
+    from xpbd_gpu.mesh import kuhn_grid
+    from xpbd_gpu.neohookean_solver import XPBDNeoHookeanSolver
+    from xpbd_gpu.sdf import PlaneSdf
+    forms = {}
+    time_one = autotune._time_graph_substeps
+
+    def spy(s, *a):
+        forms[s.scatter] = s.launch_info()["form"]
+        return time_one(s, *a)
+    monkeypatch.setattr(autotune, "_time_graph_substeps", spy)
+    m = kuhn_grid(6, 5, 7, 0.1, origin=(0.0, 0.65, 0.0), jitter=0.1, seed=2)
+    s = XPBDNeoHookeanSolver(m, PlaneSdf([0, 0, 0], [0, 1, 0], True), scatter="auto", tet_young_modulus=np.full(m.n_tets, 1e5),
+                             autotune_cache=str(tmp_path / "t.json"), block_neohookean_enable=True, frame_dt=1 / 60, dt=1 / 60,
+                             substeps_num=3, constraints_iter=10)
+    assert forms == {"atomic": 1, "gather": 0}
+    assert s.launch_info()["form"] == forms[s.scatter]
