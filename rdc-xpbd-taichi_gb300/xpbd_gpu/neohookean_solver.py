@@ -38,10 +38,11 @@ from xpbd_gpu import _native
 from xpbd_gpu.xpbd_base import XPBDSolverBase, _torch, calc_tet_volume  # noqa: F401
 
 
-# Tets up to which every 256-tet patch of a body can be resident at once (three
-# per SM): such a body's substeps run in one launch each, also with per-tet
-# materials, which then need the patch layout beside the per-tet one
-GANG_MAX_TETS = 3 * 152 * 256
+def resident_tets(device):
+    """Tets up to which every 256-tet patch of a body can be resident at once (three
+    per SM): such a body's substeps run in one launch each, also with per-tet
+    materials, which then need the patch layout beside the per-tet one."""
+    return 3 * _torch().cuda.get_device_properties(device).multi_processor_count * 256
 
 
 def calc_first_lame(E, nu):
@@ -153,7 +154,7 @@ class XPBDNeoHookeanSolver(XPBDSolverBase):
             self._tinv_mu = torch.empty(T, dtype=torch.float32, device=self._device)
             self._tinv_la = torch.empty(T, dtype=torch.float32, device=self._device)
             self.set_tet_materials(np.log(self._tet_E), self._tet_nu)
-        if self.scatter == "atomic" and self._tinv_mu is not None and self.n_tets <= GANG_MAX_TETS:
+        if self.scatter == "atomic" and self._tinv_mu is not None and self.n_tets <= resident_tets(self._device):
             self._ensure_patch_buffers()  # per-tet materials: small bodies run patch by patch all the same
         if self.scatter == "patch" and not self._ensure_patch_buffers():
             # no patch size keeps every patch within 256 vertices: per-tet variant

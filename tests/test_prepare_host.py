@@ -35,3 +35,13 @@ def test_patch_lists_cost_a_few_passes_over_the_corners(native_lib):
         np.testing.assert_array_equal(pv[voff[p]:voff[p + 1]], want)
         loc = lid[p * P:min(T, (p + 1) * P), None] >> (8 * np.arange(4, dtype=np.uint32)) & 0xff
         np.testing.assert_array_equal(want[loc], tt[p * P:(p + 1) * P])
+
+
+def test_resident_bodies_are_those_of_the_device(monkeypatch):
+    """Three patches of 256 tets per SM, as the library asks the device for it."""
+    import torch
+    from types import SimpleNamespace
+    from xpbd_gpu import neohookean_solver as n
+    for sms in (132, 148, 152, 160):
+        monkeypatch.setattr(torch.cuda, "get_device_properties", lambda device: SimpleNamespace(multi_processor_count=sms))
+        assert n.resident_tets("cuda:0") == 768 * sms
