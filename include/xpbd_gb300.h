@@ -213,6 +213,11 @@ int xpbd_read_history(void* handle, double* host_out, int32_t n, void* stream);
 int xpbd_keep_residual(void* handle, int32_t row, void* stream);
 int xpbd_kept_residual(void* handle, double* out);
 
+/* What is queued on `stream` after this call starts after the newest kept
+ * residual's copy, and so after the step before it; a stream under capture
+ * cannot wait so, and the host does. */
+int xpbd_wait_kept(void* handle, void* stream);
+
 /* Jacobi iterations run by substeps [0, n) of the last frame (or, for
  * xpbd_substep / xpbd_solve_step, by the substep whose record_base is
  * s * constraints_iter); n <= 256.  `total` (may be NULL) receives the

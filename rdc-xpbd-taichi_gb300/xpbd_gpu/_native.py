@@ -124,6 +124,7 @@ _SIGNATURES = {
     "xpbd_solve": (ctypes.c_int, [_P, ctypes.c_double, ctypes.c_double, ctypes.c_int32, _P]),
     "xpbd_read_history": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_double), ctypes.c_int32, _P]),
     "xpbd_keep_residual": (ctypes.c_int, [_P, ctypes.c_int32, _P]),
+    "xpbd_wait_kept": (ctypes.c_int, [_P, _P]),
     "xpbd_kept_residual": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_double)]),
     "xpbd_read_iterations": (ctypes.c_int, [_P, _P, ctypes.c_int32, ctypes.POINTER(ctypes.c_int64), _P]),
     "xpbd_get_rho_hat": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_double), _P]),

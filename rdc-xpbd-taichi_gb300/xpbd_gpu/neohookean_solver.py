@@ -109,6 +109,7 @@ class XPBDNeoHookeanSolver(XPBDSolverBase):
         self.rho_max = 0.99999
         self.rho_beta = 0.2
         self.prev_r_hat = None
+        self._step_stream = None  # of the last solve_step that the host did not wait for
         self._timing_events = []
         self._time_done = 0.0
         self.solve_compute_calls = 0
@@ -176,6 +177,7 @@ class XPBDNeoHookeanSolver(XPBDSolverBase):
         torch = _torch()
         if self._tinv_mu is None:
             raise RuntimeError("the solver was built without per-tet materials")
+        self._stream()
         le = torch.as_tensor(log_E, dtype=torch.float64, device=self._device).reshape(-1)
         nu_t = torch.as_tensor(nu, dtype=torch.float64, device=self._device).reshape(-1).expand(le.shape[0])
         E = torch.exp(le)
@@ -367,6 +369,12 @@ class XPBDNeoHookeanSolver(XPBDSolverBase):
             self.prev_r_hat = out.value
         return self._prev_r_hat
 
+    def _after_step(self, stream):
+        # as if the host had waited for the step's residual: the step comes before
+        # whatever is done next, on any stream
+        if self._step_stream is not None and stream != self._step_stream:
+            _native.check(self._lib.xpbd_wait_kept(self._handle, stream.cuda_stream))
+
     @prev_r_hat.setter
     def prev_r_hat(self, value):
         self._prev_r_hat = value
@@ -395,12 +403,14 @@ class XPBDNeoHookeanSolver(XPBDSolverBase):
         if self.cheb_enable and n_it > 0:
             if self.stop_mode or self.monitor_convergence or _torch().cuda.is_current_stream_capturing():
                 self.prev_r_hat = float(self.read_history(self.constraints_iter)[n_it - 1, 0])
+                self._step_stream = None
             else:
                 # the copy is queued here and waited for where the value is read: the
                 # host stays ahead of the device over a loop of steps (5 substeps of a
                 # 12x11x10-cell body with their two state copies: 873-938 -> 650 us)
                 _native.check(self._lib.xpbd_keep_residual(self._handle, n_it - 1, self._stream()))
                 self._r_hat_kept = True
+                self._step_stream = _torch().cuda.current_stream(self._device)
 
     def solve(self):
         """neohookean_solver.py:562-587: one frame."""

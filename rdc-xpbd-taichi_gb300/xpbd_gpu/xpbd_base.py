@@ -109,6 +109,7 @@ class CellField:
     def fill(self, value):
         if value != 0.0:
             raise ValueError("only fill(0.0) is supported")
+        self._s._stream()
         self._s._lam.zero_()
 
 
@@ -406,9 +407,17 @@ class XPBDSolverBase:
 
     # -- device access helpers -------------------------------------------------
     def _stream(self):
-        return _torch().cuda.current_stream(self._device).cuda_stream
+        """The current stream, behind a solve_step that was left queued on another one.
+        Called before anything that touches the device state."""
+        st = _torch().cuda.current_stream(self._device)
+        self._after_step(st)
+        return st.cuda_stream
+
+    def _after_step(self, stream):
+        pass
 
     def _cell_array(self, t):
+        self._stream()
         a = t.detach().cpu().numpy()
         out = np.empty_like(a)
         out[self._tperm] = a
@@ -432,11 +441,13 @@ class XPBDSolverBase:
         a = arr if isinstance(arr, torch.Tensor) else torch.from_numpy(np.ascontiguousarray(arr, dtype=np.float32))
         if tuple(a.shape) != (self.n_verts, 3):
             raise ValueError("expected shape (%d, 3), got %s" % (self.n_verts, tuple(a.shape)))
+        st = self._stream()
         self._stage.copy_(a, non_blocking=True)
-        _native.check(self._lib.xpbd_import_vec3(self._handle, field_id, self._stage.data_ptr(), self._stream()))
+        _native.check(self._lib.xpbd_import_vec3(self._handle, field_id, self._stage.data_ptr(), st))
 
     def _set_inv_m(self, inv_m):
         torch = _torch()
+        self._stream()
         self._host_inv_m = inv_m.copy()
         w = torch.from_numpy(inv_m[self._vperm].astype(np.float32)).to(self._device)
         self._x4[:, 3] = w
