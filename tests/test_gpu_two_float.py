@@ -72,3 +72,15 @@ def test_operations(ops):
 def test_narrow_rounds_like_a_conversion(ops):
     a = np.concatenate([_doubles(20000, 7, -140, 126), 1.0 + np.arange(-64, 64) * 2.0 ** -25, [0.0, np.inf, -np.inf]])
     np.testing.assert_array_equal(ops(a)["narrow"], a.astype(np.float32))
+
+
+def test_every_float_widens_exactly(ops):
+    """Denormal floats too: a material adjoint of 1e-40 is a summand like any other."""
+    r = np.random.default_rng(8)
+    f = np.concatenate([r.integers(0, 1 << 32, 20000, dtype=np.uint64).astype(np.uint32).view(np.float32),
+                        np.arange(1, 2000, dtype=np.uint32).view(np.float32),
+                        np.array([0.0, -0.0, np.inf, -np.inf, 1e-40, -1e-45, 1.17549435e-38], dtype=np.float32)])
+    f = f[~np.isnan(f)]
+    w = ops(np.ones(len(f)), f=f)["wide"]
+    np.testing.assert_array_equal(w, f.astype(np.float64))
+    np.testing.assert_array_equal(np.signbit(w), np.signbit(f))
