@@ -114,3 +114,15 @@ def test_infinite_residual_meets_its_target(name):
     s.solve()
     assert np.isposinf(rows()[:, 0, 0]).all()
     assert (np.atleast_2d(s.iterations_per_substep()) == 1).all()
+
+
+@pytest.mark.parametrize("name", FORMS)
+def test_recorded_residuals_have_fp64_digits(name):
+    """r_hat is the FP64 sum over the tet count: its last two bits are set as often as
+    not.  A two-float value of 48 bits has them clear unless its parts lie apart."""
+    _, make = FORMS[name]
+    s, rows, _ = make(substeps_num=4)
+    s.solve()
+    r = rows()[:, :, 0].ravel()
+    low = np.ascontiguousarray(r).view(np.uint64) & np.uint64(3)
+    assert len(r) >= 160 and (low != 0).mean() > 0.5
