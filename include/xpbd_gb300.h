@@ -11,7 +11,7 @@
  *  - Every function returns an int status (XPBD_OK == 0).
  *  - Device buffers are allocated by the caller (e.g. torch CUDA tensors) and
  *    passed as raw pointers; the library never frees them.  The library owns
- *    only a small per-solver block of device state (SDF table, FP64 Chebyshev
+ *    only a small per-solver block of device state (SDF table, Chebyshev
  *    state, per-iteration history), released by xpbd_destroy.
  *  - `stream` is a cudaStream_t passed as void*; NULL means the legacy default
  *    stream.  All work is stream-ordered; no entry point synchronises unless
@@ -243,7 +243,7 @@ enum xpbd_kernel_class {
   XPBD_K_BEGIN = 0,    /* predict + SDF (V) */
   XPBD_K_PROJECT = 1,  /* Neo-Hookean projection + Jacobi scatter (T) */
   XPBD_K_GATHER = 2,   /* deterministic vertex gather (V) */
-  XPBD_K_RESIDUAL = 3, /* residual / monitoring sweep + FP64 scalars (T) */
+  XPBD_K_RESIDUAL = 3, /* residual / monitoring sweep and its sums (T) */
   XPBD_K_UPDATE = 4,   /* post_solve + Chebyshev mix (V) */
   XPBD_K_END = 5,      /* advance (V) */
   XPBD_K_COUNT = 6
@@ -253,8 +253,9 @@ enum xpbd_kernel_class {
  * on its stream.  With use_graph, xpbd_solve replays a frame graph that
  * carries those events as event record nodes, and waits for the previous
  * profiled replay before launching the next; without it the launches are
- * direct.  (The reference's counterpart is the host perf_counter brackets of
- * solve_step, neohookean_solver.py:454-560.) */
+ * direct.  A body or batch whose substeps are single launches (below) runs
+ * launch per phase while profiled.  (The reference's counterpart is the host
+ * perf_counter brackets of solve_step, neohookean_solver.py:454-560.) */
 int xpbd_set_profiling(void* handle, int32_t enable);
 
 /* How the next frame's substeps run with the parameters in force.  form 0: one

@@ -10,7 +10,7 @@ Chebyshev state (``rho_hat`` persists across substeps and frames).
 Every substep runs on the GPU as hand-written sm_103a kernels
 (``libxpbd_gb300.so``, ``include/xpbd_gb300.h``).  The residual r_hat, the
 spectral-radius estimate rho_hat and the omega recurrence are evaluated on
-the device in FP64, so a frame needs no host round trip; ``solve()`` replays
+the device (two-float arithmetic and FP64), so a frame needs no host round trip; ``solve()`` replays
 one cached CUDA graph per frame.  With ``monitor_convergence`` the frame is
 driven substep by substep so that ``convergence_callback`` fires after each
 substep, as in the reference (:574-583).
