@@ -197,13 +197,13 @@ __global__ void __launch_bounds__(256) ka_chain(D d, Tape tp, Adj a, ChainPrm c)
 }
 
 // Reverse of advance: live vertices x' = x~_K, v' = (x~_K - x) e / dt; pinned
-// vertices keep x and v.
+// vertices keep x and v.  Which are pinned the tape says, as the forward ran.
 template <class D>
-__global__ void __launch_bounds__(256) ka_end(D d, Adj a, float e_over_dt) {
+__global__ void __launch_bounds__(256) ka_end(D d, Tape tp, Adj a, float e_over_dt) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= adj_verts(d)) return;
   const float4 gx = a.gx[i], gv = a.gv[i];
-  if (d.x[i].w > 0.f) {
+  if (tp.xpre[i].w > 0.f) {
     a.abuf[0][i] = make_float4(gx.x + gv.x * e_over_dt, gx.y + gv.y * e_over_dt, gx.z + gv.z * e_over_dt, 0.f);
     a.gx[i] = make_float4(-gv.x * e_over_dt, -gv.y * e_over_dt, -gv.z * e_over_dt, 0.f);
     a.gv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(256) ka_begin(D d, Tape tp, Adj a, int src, in
     gb.z += q.z;
   }
   const float4 pre = tp.xpre[i];
-  if (d.x[i].w > 0.f) {
+  if (pre.w > 0.f) {
     const float3 vel = f3(tp.v1[i]);
     for (int s = d.n_sdf - 1; s >= 0; --s) {
       // positions entering SDF s: replay the list up to s
